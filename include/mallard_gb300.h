@@ -321,7 +321,8 @@ int mgpu_calc_dt_noalloc(mgpu_ctx* ctx, double cfl, double* dt_device, double* s
  * smoothness indicators of every variable whose predicted class reaches
  * the probability threshold in the cell and in all its face neighbours, and
  * the cell evaluates only the stencils its variables need; any other
- * variable runs full TENO. */
+ * variable runs full TENO.  Calls on one selector from several threads run
+ * one after the other. */
 #define MGPU_SEL_INPUTS 96
 #define MGPU_SEL_OUTPUTS 32
 #define MGPU_SEL_CLASSES 8

@@ -7,9 +7,11 @@
 // the cut-off weights fixed) computed by the FP64 kernels on the solver's
 // own states.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <random>
 #include <vector>
@@ -21,6 +23,9 @@
 using namespace mgpu;
 
 struct mgpu_selector {
+    // every entry that touches the selector holds it: the stream, the weights
+    // and the buffers below serve one call at a time
+    std::mutex lock;
     int device = 0;
     cudaStream_t stream = nullptr;
     std::vector<float> params;  // host copy, authoritative between calls
@@ -31,13 +36,15 @@ struct mgpu_selector {
     // dataset
     DevArray<float> X;
     DevArray<uint8_t> Y;
-    size_t n = 0, cap = 0;
+    std::atomic<size_t> n{0};  // read without the lock by mgpu_selector_dataset_size
+    size_t cap = 0;
     // batch work
     size_t wb = 0;
     DevArray<float> Xb, Z1, A1, Z2, A2, Z3, dZ3, dA, dZ, work, part;
     DevArray<uint8_t> Yb;
     DevArray<uint32_t> perm;
-    // inference over host rows: rows, logits, predictions
+    // inference over host rows: rows, logits, predictions; kept for the next
+    // call, up to KEEP_ROWS rows
     DevArray<float> infer_x, infer_l;
     DevArray<uint8_t> infer_p;
     DevArray<unsigned> err;
@@ -81,6 +88,9 @@ std::vector<uint8_t> weight_image(const std::vector<float>& p) {
     std::memcpy(&img[off], p.data() + sel::OFF_B3, sel::OUT * 4);
     return img;
 }
+
+// Rows whose inference buffers (516 bytes each) outlive the call: 135 MB.
+constexpr size_t KEEP_ROWS = (size_t)1 << 18;
 
 struct DeviceGuard {
     int prev = -1;
@@ -252,6 +262,7 @@ void mgpu_selector_destroy(mgpu_selector* s) {
 int mgpu_selector_get_params(mgpu_selector* s, float* params) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (!params) throw ArgFail("null argument");
         std::memcpy(params, s->params.data(), s->params.size() * 4);
         return MGPU_OK;
@@ -261,6 +272,7 @@ int mgpu_selector_get_params(mgpu_selector* s, float* params) {
 int mgpu_selector_set_params(mgpu_selector* s, const float* params) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (!params) throw ArgFail("null argument");
         DeviceGuard g(s->device);
         std::memcpy(s->params.data(), params, s->params.size() * 4);
@@ -285,6 +297,7 @@ int mgpu_selector_dataset_size(const mgpu_selector* s, uint64_t* n) {
 
 int mgpu_selector_clear(mgpu_selector* s) {
     if (int rc = need_sel(s)) return rc;
+    std::lock_guard<std::mutex> hold(s->lock);
     s->n = 0;
     return MGPU_OK;
 }
@@ -292,6 +305,7 @@ int mgpu_selector_clear(mgpu_selector* s) {
 int mgpu_selector_add_samples(mgpu_selector* s, const float* X, const uint8_t* Y, uint64_t n) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if ((!X || !Y) && n) throw ArgFail("null argument");
         for (uint64_t i = 0; i < n * sel::NV; ++i)
             if (Y[i] >= sel::NCLS) throw ArgFail("class label out of range");
@@ -308,6 +322,7 @@ int mgpu_selector_add_samples(mgpu_selector* s, const float* X, const uint8_t* Y
 int mgpu_selector_get_samples(mgpu_selector* s, uint64_t first, uint64_t n, float* X, uint8_t* Y) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (first + n > s->n) throw ArgFail("sample range outside the dataset");
         DeviceGuard g(s->device);
         if (X) ck(cudaMemcpyAsync(X, s->X.p + first * sel::IN, n * sel::IN * 4, cudaMemcpyDeviceToHost, s->stream), "D2H");
@@ -321,6 +336,7 @@ int mgpu_selector_harvest(mgpu_selector* s, mgpu_ctx* ctx, double keep_central, 
     if (int rc = need_sel(s)) return rc;
     if (int rc = need_ready(ctx)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (ctx->cfg.recon != MGPU_RECON_TENO || ctx->K != 10 || ctx->cfg.teno_variant == MGPU_TENO_REFERENCE ||
             ctx->single())
             throw Unsupported("harvest needs an FP64 context with corrected or robust TENO at p = 3");
@@ -356,6 +372,7 @@ int mgpu_selector_harvest(mgpu_selector* s, mgpu_ctx* ctx, double keep_central, 
 int mgpu_selector_gradient(mgpu_selector* s, const float* X, const uint8_t* Y, uint32_t n, float* grad, float* loss) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (!X || !Y || !grad || n == 0) throw ArgFail("null or empty argument");
         DeviceGuard g(s->device);
         ensure_batch(s, n);
@@ -380,6 +397,7 @@ int mgpu_selector_train(mgpu_selector* s, uint32_t epochs, uint32_t batch, float
                         float* epoch_loss) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (s->n == 0) throw ArgFail("empty dataset");
         if (batch == 0 || epochs == 0) throw ArgFail("batch and epochs must be positive");
         if (s->n > 0xffffffffull) throw ArgFail("dataset too large");
@@ -427,10 +445,21 @@ int mgpu_selector_infer(mgpu_selector* s, const float* X, uint32_t n, float thr_
                         float* logits, uint8_t* pred) {
     if (int rc = need_sel(s)) return rc;
     return guarded([&] {
+        std::lock_guard<std::mutex> hold(s->lock);
         if (!X || n == 0) throw ArgFail("null or empty argument");
         DeviceGuard g(s->device);
         refresh_image(s);
         ck(sel::mlp_prepare(), "cudaFuncSetAttribute");
+        struct Bound {  // given back after a call with more rows, however it ends
+            mgpu_selector* s;
+            ~Bound() {
+                if (s->infer_x.n <= KEEP_ROWS * sel::IN) return;
+                cudaStreamSynchronize(s->stream);
+                s->infer_x.release();
+                s->infer_l.release();
+                s->infer_p.release();
+            }
+        } bound{s};
         // kept for the next call, grown when a larger one comes
         DevArray<float>&dx = s->infer_x, &dl = s->infer_l;
         DevArray<uint8_t>& dp = s->infer_p;
@@ -466,6 +495,7 @@ int mgpu_set_selector(mgpu_ctx* ctx, mgpu_selector* s, float thr_central, float 
         if (!ctx->single() || ctx->K != 10) throw Unsupported("the learned selector drives the FP32 form at p = 3");
         if (ctx->cfg.device != s->device) throw ArgFail("selector and context are on different devices");
         if (thr_central > 1.0f) throw ArgFail("central threshold above 1");
+        std::lock_guard<std::mutex> hold(s->lock);
         DeviceGuard g(s->device);
         refresh_image(s);
         ck(sel::mlp_prepare(), "cudaFuncSetAttribute");
