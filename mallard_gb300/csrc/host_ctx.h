@@ -52,7 +52,11 @@ struct DevArray {
     }
     void upload(const std::vector<T>& v) {
         alloc(v.size());
-        if (!v.empty()) ck(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy H2D");
+        if (v.empty()) return;
+        ck(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "cudaMemcpy H2D");
+        // a copy from pageable memory may return with its last piece still on
+        // the way, on the legacy stream as well
+        ck(cudaStreamSynchronize(cudaStreamLegacy), "cudaStreamSynchronize");
     }
     size_t bytes() const { return n * sizeof(T); }
 };

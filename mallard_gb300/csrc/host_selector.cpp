@@ -503,7 +503,10 @@ int mgpu_set_selector(mgpu_ctx* ctx, mgpu_selector* s, float thr_central, float 
         if (!ctx->pred.p) ctx->pred.alloc((size_t)ctx->N * 4);
         if (!ctx->trusted.p) ctx->trusted.alloc((size_t)ctx->N * 4);
         if (!ctx->sel_err.p) ctx->sel_err.alloc(1);
-        ck(cudaMemcpy(ctx->sel_wimg.p, s->d_wimg.p, sel::WEIGHT_IMAGE_BYTES, cudaMemcpyDeviceToDevice), "D2D");
+        ck(cudaMemcpyAsync(ctx->sel_wimg.p, s->d_wimg.p, sel::WEIGHT_IMAGE_BYTES, cudaMemcpyDeviceToDevice, ctx->stream),
+           "D2D");
+        // the selector's image may change once the lock is gone
+        ck(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
         ctx->sel_thr_central = thr_central;
         ctx->sel_thr_directional = thr_directional;
         ctx->sel_on = true;
