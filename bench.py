@@ -120,7 +120,7 @@ def parse():
                          "crosses about 0.12 of a cell per step, so 4 steps stay inside the neighbour check's "
                          "one-cell margin)")
     ap.add_argument("--shape", type=int, default=-1,
-                    help="fix the FP32 reconstruction's launch shape (0-7) instead of autotuning it")
+                    help="fix the FP32 reconstruction's launch shape (0-10) instead of autotuning it")
     ap.add_argument("--cpu-sample-n", type=int, default=CPU_SAMPLE_N)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     return ap.parse_args()
@@ -366,7 +366,8 @@ def autotune(s, args, U0, W0):
     return {"chosen_shape": shape, "ms_per_shape": [round(x, 4) for x in tms],
             "shapes": "0: 128 thr/<=128 regs, 1: 128/<=80, 2: 128/<=64, 3: 256/<=64, "
                       "bulk copies to shared memory: 4 staged, 4 warps/<=72 regs; 5-7 proof of the central "
-                      "decision, 2, 1 and 3 warps (below 100,000 cells 4-7 all staged)"}
+                      "decision, 2, 1 and 3 warps; 8-10 staged, 4 warps/<=80 regs, 2 warps, 1 warp (below "
+                      "100,000 cells 4-7 all staged and 8-10 the same as 4-6)"}
 
 
 def time_form(m, args, form, U0, W0, device, selector, barrier=None, clocks=None):

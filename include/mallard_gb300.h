@@ -437,19 +437,22 @@ int mgpu_enable_kernel_timing(mgpu_ctx* ctx, int enable);
 int mgpu_kernel_times(mgpu_ctx* ctx, double* ms, uint32_t* launches);
 /* Autotuner: times each launch shape of the reconstruction kernel (FP32
  * form at p = 3: 0-2 128-thread blocks with at most 128, 80 or 64 registers
- * per thread, 3 256-thread blocks with 64, 4-7 kernels whose warps copy
+ * per thread, 3 256-thread blocks with 64, 4-10 kernels whose warps copy
  * their tile's tables into shared memory with bulk async copies: from
- * 100,000 cells 4 is the staged form (one stencil slot per warp, 4 warps per
- * block, at most 72 registers) and 5-7 the proof form (cells whose central
- * decision is proven, then the others in a second launch) with 2, 1 and 3
- * warps per block; below, all four are the staged form, with 4 warps per
- * block and at most 80 registers, then 2, 1 and 4 with at most 72) on the
- * current state, three launches each after a warm-up, and keeps the fastest
- * for later launches.  Until then shape 7 (FP32 form at p = 3).
+ * 100,000 cells 4 and 8-10 are the staged form (one stencil slot per warp; 4
+ * warps per block and at most 72 registers, 4 warps and 80, 2 warps and 1
+ * warp with 72) and 5-7 the proof form (cells whose central decision is
+ * proven, then the others in a second launch) with 2, 1 and 3 warps per
+ * block; below, 4-7 are the staged form, with 4 warps per block and at most
+ * 80 registers, then 2, 1 and 4 with at most 72, and 8-10 the same as 4-6)
+ * on the current state, three launches each after a warm-up, and keeps the
+ * fastest for later launches.  Until then shape 7 (FP32 form at p = 3): the
+ * fastest from 100,000 cells but where a selector is confident nearly
+ * everywhere, so a learned run should be tuned on a state of its flow.
  * ms[MGPU_AUTOTUNE_SHAPES] receives the average time per shape (0 where not
  * applicable), best the chosen shape.  Both may be NULL.  Other forms have
  * a single shape. */
-#define MGPU_AUTOTUNE_SHAPES 8
+#define MGPU_AUTOTUNE_SHAPES 11
 int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best);
 /* Fix the reconstruction's launch shape (as mgpu_autotune numbers them);
  * every shape gives the same results. */

@@ -25,7 +25,7 @@ BC_TYPES = {"symmetry": 0, "extrapolation": 1, "wall_adiabatic": 2, "upt": 3, "p
 TENO_VARIANTS = {"reference": 0, "corrected": 1, "robust": 2}
 PRECISIONS = {"fp64": 0, "fp64_fast": 1, "fp32": 2}
 VISC_GRADIENTS = {"recon": 0, "green_gauss": 1}
-AUTOTUNE_SHAPES = 8  # MGPU_AUTOTUNE_SHAPES
+AUTOTUNE_SHAPES = 11  # MGPU_AUTOTUNE_SHAPES
 
 TENO_FIELDS = {
     "offsets_stencil_groups": (0, "uint32"),

@@ -242,9 +242,11 @@ MGPU_DECLARE_TENO_FLUX
 namespace f32 {
 // shape: launch shape 0..3 (128-thread blocks with at most 128, 80 or 64
 // registers, or 256-thread blocks with 64; p = 3 only, other orders use
-// shape 0) or 4..7, forms that copy each tile's table blocks
+// shape 0) or 4..10, forms that copy each tile's table blocks
 // into shared memory with cp.async.bulk; chosen by the autotuner
 constexpr int TENO32_SHAPES = MGPU_AUTOTUNE_SHAPES;
+// cells from which shapes 5-7 are the proof form and 8-10 not the same as 4-6
+constexpr int PROOF_MIN_CELLS = 100000;
 // the batched reconstruction has shape 6, the proof form, and shapes 7 and 8:
 // one CTA of 4 or 8 warps per mesh tile, its tables resident in shared memory
 // for all cases

@@ -1352,15 +1352,16 @@ cudaError_t teno_proof1(const TenoArgs& a, const float* U, float* fv, uint8_t* m
 
 // Launch shapes the autotuner chooses from: (block size, minimum resident
 // blocks per SM), i.e. register caps of 128, 80 and 64 per thread; shapes
-// 4-7 copy their tables into shared memory (p = 3).  From PROOF_MIN_CELLS: 4
-// the staged kernel, one stencil slot and at most 72 registers, 4 warps per
-// block; 5-7 the proof form with 2, 1 and 3 warps.  Below: the staged kernel
-// with 4 warps and at most 80 registers, then 2, 1 and 4 with at most 72.
+// 4-10 copy their tables into shared memory (p = 3).  From PROOF_MIN_CELLS: 4
+// and 8-10 the staged kernel, one stencil slot, with 4 warps per block and at
+// most 72 registers, then 4 warps and 80, 2 warps and 1 warp with 72; 5-7 the
+// proof form with 2, 1 and 3 warps.  Below, 4-7 are the staged kernel with 4
+// warps and at most 80 registers, then 2, 1 and 4 with at most 72, and 8-10
+// the same as 4-6.
 // Below this many cells the tables of a pass come from L2 and the second launch costs
 // more than the proof saves (plain form, us a launch, proof against staged:
 // 66,000 cells 46 against 42, 131,000 70 against 74, 262,000 113 against 136,
 // 524,000 191 against 256).
-constexpr int PROOF_MIN_CELLS = 100000;
 template <int K, int M, int NQ, bool SEL, bool VG>
 cudaError_t teno_go(const TenoArgs& a, const float* U, float* fv, uint8_t* masks, const uint8_t* pred, int shape,
                     cudaStream_t s) {
@@ -1372,18 +1373,18 @@ cudaError_t teno_go(const TenoArgs& a, const float* U, float* fv, uint8_t* masks
     }
     if constexpr (K == 10 && M == 20 && NQ == 2) {
         if (a.cert && a.n_cells >= PROOF_MIN_CELLS) {
-            // shape 4 keeps the staged kernel: where the selector is confident
-            // nearly everywhere it has a launch and half a table less to wait for
-            // (1024^2, 97% of the cells: 394 us a launch against 422; 69%: 637
-            // against 490)
+            // shapes 4 and 8-10 keep the staged kernel: where the selector is
+            // confident nearly everywhere it has a launch and half a table less to
+            // wait for (1024^2, 97% of the cells: 394 us a launch against 422; 69%:
+            // 637 against 490)
             if (shape == 4) return teno_staged1<K, M, NQ, SEL, 1, 4, 7, VG>(a, U, fv, masks, pred, s);
             if (shape == 5) return teno_proof1<K, M, NQ, SEL, 2, 13, VG>(a, U, fv, masks, pred, s);
             if (shape == 6) return teno_proof1<K, M, NQ, SEL, 1, 24, VG>(a, U, fv, masks, pred, s);
             if (shape == 7) return teno_proof1<K, M, NQ, SEL, 3, 8, VG>(a, U, fv, masks, pred, s);
         }
-        if (shape == 4) return teno_staged1<K, M, NQ, SEL, 1, 4, 6, VG>(a, U, fv, masks, pred, s);
-        if (shape == 5) return teno_staged1<K, M, NQ, SEL, 1, 2, 14, VG>(a, U, fv, masks, pred, s);
-        if (shape == 6) return teno_staged1<K, M, NQ, SEL, 1, 1, 28, VG>(a, U, fv, masks, pred, s);
+        if (shape == 4 || shape == 8) return teno_staged1<K, M, NQ, SEL, 1, 4, 6, VG>(a, U, fv, masks, pred, s);
+        if (shape == 5 || shape == 9) return teno_staged1<K, M, NQ, SEL, 1, 2, 14, VG>(a, U, fv, masks, pred, s);
+        if (shape == 6 || shape == 10) return teno_staged1<K, M, NQ, SEL, 1, 1, 28, VG>(a, U, fv, masks, pred, s);
         if (shape == 7) return teno_staged1<K, M, NQ, SEL, 1, 4, 7, VG>(a, U, fv, masks, pred, s);
     }
     return cudaErrorInvalidValue;

@@ -1244,7 +1244,9 @@ int mgpu_kernel_times(mgpu_ctx* ctx, double* ms, uint32_t* launches) {
 int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best) {
     if (int rc = need_ready(ctx)) return rc;
     return guarded([&] {
-        const int n = ctx->single() && ctx->K == 10 ? f32::TENO32_SHAPES : 1;
+        // shapes 8-10 are 4-6 again where no proof form takes their place
+        const bool proof = ctx->teno.cert && ctx->N >= (uint32_t)f32::PROOF_MIN_CELLS;
+        const int n = !(ctx->single() && ctx->K == 10) ? 1 : (proof ? f32::TENO32_SHAPES : 8);
         std::vector<double> t(f32::TENO32_SHAPES, 0.0);
         cudaEvent_t a, b;
         ck(cudaEventCreate(&a), "cudaEventCreate");
