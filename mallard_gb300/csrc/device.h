@@ -98,6 +98,10 @@ struct TenoArgs {
     float2* vgb;
 };
 
+// Face points up to which the FP64 flux runs with one lane per side (two warps
+// of points on each of the 608 schedulers); above, one lane per point.
+constexpr long long FLUX_SIDE_POINTS = 608ll * 2 * 32;
+
 struct FluxArgs {
     int n_faces;            // faces that carry a flux
     const int2* lr;         // internal cell ids; y = -1 on boundary faces

@@ -155,6 +155,7 @@ int mgpu_batch_finalize(mgpu_batch* b) {
             mgpu_config cfg = b->cfg;
             if (mgpu_create(b->meshes[g], &cfg, &c) != MGPU_OK) throw ArgFail(mgpu_last_error());
             b->groups.emplace_back(c, destroy_ctx);
+            c->in_batch = true;
             for (const BcHost& h : b->bcs) {
                 int nd = h.type == MGPU_BC_UPT ? 4 : (h.type == MGPU_BC_P_OUT ? 1 : 0);
                 if (mgpu_add_boundary(c, h.zone, h.type, nd ? h.data : nullptr, nd) != MGPU_OK)

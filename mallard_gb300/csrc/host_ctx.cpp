@@ -232,8 +232,10 @@ void mgpu_ctx::build_cert(const TenoTables& t) {
         Up.alloc((size_t)N * 4);
         Utp.alloc((size_t)N * 4);
     }
-    hard.alloc(N);
-    hard_n.alloc(2);
+    if (!in_batch) {  // a batch has one list for all its meshes
+        hard.alloc(N);
+        hard_n.alloc(2);
+    }
     a.n_cells = (int)N;
     a.M = M;
     a.K = K;
@@ -641,7 +643,8 @@ void mgpu_ctx::build() {
         teno.phi_tab4 = phi_tab4.p;
         teno.cface = cface.p;
         teno.smask = smask.p;
-        if (!f32 || K == 10) build_cert(t);
+        // the FP32 form alone reads them from PROOF_MIN_CELLS only
+        if (!f32 || (K == 10 && (in_batch || N >= (uint32_t)f32::PROOF_MIN_CELLS))) build_cert(t);
         // compulsory bytes of one reconstruction launch: tables, shapes (the
         // FP32 form: a 2-byte code per cell), face slots, the state gathered
         // once per cell, face states written
@@ -704,7 +707,7 @@ void mgpu_ctx::build() {
         Ut32.alloc((size_t)N * 4);
     }
     else fv.alloc((size_t)F_real * nq * 8);
-    if (cfg.recon == MGPU_RECON_FO) sides.alloc((size_t)N * 8);
+    if (cfg.recon == MGPU_RECON_FO && (long long)F_flux * nq > FLUX_SIDE_POINTS) sides.alloc((size_t)N * 8);
     G.alloc((size_t)F_flux * 4);
     scal.alloc(2);
     flags.alloc(1);

@@ -77,6 +77,7 @@ struct mgpu_ctx {
     HostMesh mesh;
     std::vector<BcHost> bcs;
     bool finalized = false;
+    bool in_batch = false;  // one mesh of an mgpu_batch
     GasParams gas{};
     BcTable bct{};
     int nq = 1, K = 0, M = 0;
