@@ -459,7 +459,8 @@ int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best);
 int mgpu_set_launch_shape(mgpu_ctx* ctx, int shape);
 /* Algorithmic bytes one reconstruction and one full stage move when every
  * cell runs all its stencils, from the actual table sizes (a cell whose
- * central decision is proven reads less). */
+ * central decision is proven reads less); a first-order stage holds no
+ * reconstruction. */
 int mgpu_traffic_model(mgpu_ctx* ctx, double* recon_bytes, double* stage_bytes);
 /* A copy of one reconstruction table as the kernels read it (tiled layout,
  * library cell order), to compare the GPU and host table builds.  dst null:

@@ -816,10 +816,14 @@ void mgpu_ctx::build() {
         }
     }
     // compulsory bytes of one stage: reconstruction + flux (face states in,
-    // G out, face geometry) + update (G gathered, state in/out)
-    const double flux_b = (double)F_flux * (nq * 64 + 32 + 8 + 16 + 8 + 1);
+    // G out, face geometry) + update (G gathered, state in/out).  First order
+    // has no reconstruction in a stage: the flux reads the cells' averages, on
+    // a large mesh by way of a row of 64 bytes per cell.
+    const bool fo = cfg.recon == MGPU_RECON_FO;
+    const double states_b = fo ? (double)N * (sides.p ? 32 + 2 * 64 : 32) : (double)F_flux * nq * 64;
+    const double flux_b = states_b + (double)F_flux * (32 + 8 + 16 + 8 + 1);
     const double upd_b = (double)N * (16 + 8 + 32 * 4) + (double)F_flux * 32 * 2;
-    stage_bytes = recon_bytes + flux_b + upd_b;
+    stage_bytes = (fo ? 0.0 : recon_bytes) + flux_b + upd_b;
     // the launch shape until mgpu_autotune or a fixed shape says otherwise:
     // the bulk-copied tables are never slower than the direct kernel and from
     // 32,768 cells faster (us a launch, shape 7 against 0: 8,192 cells 12.5
