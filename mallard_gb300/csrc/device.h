@@ -69,7 +69,7 @@ struct TenoArgs {
     double oi[KR_MAX * KR_MAX];   // oscillation indicator without dof 0, row-major (K-1)^2
     double oi2[KR_MAX * KR_MAX];  // same, upper triangle with doubled off-diagonals (fast form)
     float oi2f[KR_MAX * KR_MAX];  // oi2 in FP32 (FP32-bulk form)
-    unsigned* err;                // status word: bit 2 when a bounded wait ran out (staged FP32 form)
+    unsigned* err;                // status word: STATUS_WAIT (forms that copy into shared memory)
     // robust TENO variant: per cell 1 if it has a boundary face
     const uint8_t* bcell;         // null unless the variant is MGPU_TENO_ROBUST
     // Proof of the central decision (teno_cert.cuh): per directional stencil
@@ -97,6 +97,10 @@ struct TenoArgs {
     float4* vga;
     float2* vgb;
 };
+
+// Bit of the status word (mgpu_status, mgpu_batch_status): a bounded device
+// wait ran out.
+constexpr unsigned STATUS_WAIT = 4u;
 
 // Face points up to which the FP64 flux runs with one lane per side (two warps
 // of points on each of the 608 schedulers); above, one lane per point.

@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) teno32_staged_kernel(const T
     if (!src.ok) {
         // a wait ran out: flag it and give every copy still pending on this
         // warp's stage one more bounded wait before the shared memory goes
-        if (lane32 == 0 && err) atomicOr(err, 1u);
+        if (lane32 == 0 && err) atomicOr(err, STATUS_WAIT);
         for (int i = 0; i <= NSLOT; ++i) {
             const int uses = i == NSLOT ? 1 : (i < src.issued ? (src.issued - i + NSLOT - 1) / NSLOT : 0);
             if (uses > 0) mbar_wait(src.bar(i), (unsigned)(uses - 1) & 1u);
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) teno32_proof_kernel(const Te
     if (!ok) {
         // a wait ran out: flag it and give the copies one more bounded wait
         // before the shared memory goes
-        if (lane32 == 0 && err) atomicOr(err, 1u);
+        if (lane32 == 0 && err) atomicOr(err, STATUS_WAIT);
         mbar_wait(bar, 0u);
         if (SEL && want) mbar_wait(bar + 1, 0u);
         if (issued) mbar_wait(bar + 2, 0u);
@@ -1498,7 +1498,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) teno32_batch_staged_kernel(c
     teno32_cell<K, M, NQ, false, false>(a, U, b.fv, nullptr, nullptr, cell, v, 0xffffffffu,
                                  IxB{b.ubase[gi], b.fbase[gi], C, cs}, src, cell < b.n_cells[gi]);
     if (!src.ok) {
-        if (lane32 == 0) atomicOr(b.flags + gc, 4u);
+        if (lane32 == 0) atomicOr(b.flags + gc, STATUS_WAIT);
         for (int i = 0; i <= NSLOT; ++i) {
             const int uses = i == NSLOT ? 1 : (i < src.issued ? (src.issued - i + NSLOT - 1) / NSLOT : 0);
             if (uses > 0) mbar_wait(src.bar(i), (unsigned)(uses - 1) & 1u);
@@ -1572,7 +1572,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) teno32_batch_resident_kernel
     const unsigned C = b.C[gi];
     if (!ok) {
         if (threadIdx.x == 0)
-            for (unsigned cs = 0; cs < C; ++cs) atomicOr(b.flags + b.case0[gi] + cs, 4u);
+            for (unsigned cs = 0; cs < C; ++cs) atomicOr(b.flags + b.case0[gi] + cs, STATUS_WAIT);
         mbar_wait(bar, 0);
         return;
     }
@@ -1621,7 +1621,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) teno32_batch_proof_kernel(co
     const unsigned C = b.C[gi];
     if (!ok) {
         if (threadIdx.x == 0)
-            for (unsigned cs = 0; cs < C; ++cs) atomicOr(b.flags + b.case0[gi] + cs, 4u);
+            for (unsigned cs = 0; cs < C; ++cs) atomicOr(b.flags + b.case0[gi] + cs, STATUS_WAIT);
         mbar_wait(bar, 0u);
         mbar_wait(bar + 2, 0u);
         return;

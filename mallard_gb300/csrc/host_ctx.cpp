@@ -1211,7 +1211,7 @@ int mgpu_status(mgpu_ctx* ctx, uint32_t* flags) {
         ck(cudaMemcpyAsync(&h, ctx->flags.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream), "D2H");
         ck(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
         if (flags) *flags = h;
-        if (h & 4u) {
+        if (h & STATUS_WAIT) {
             set_error("a bounded device wait ran out");
             return MGPU_ERR_TIMEOUT;
         }
