@@ -256,8 +256,10 @@ int mgpu_batch_finalize(mgpu_batch* b) {
         // says otherwise: the staged kernel for a small batch (50,000 cells: 38
         // us a launch against 62 direct), else tables resident in shared memory,
         // with the central-decision proof where a case is large enough for its
-        // jumps to cover little of it (1.66M cells, 52,000 a case: 770 us
-        // against 855 without and 1,427 direct; 8,192 a case: 696 against 486)
+        // jumps to cover little of it (random quadrant states after 30 steps,
+        // proof against resident, us a launch: 12,800 cells a case 616 and 526,
+        // 18,432 610 and 565, 25,088 638 and 634, 32,768 618 and 641, 100,352
+        // 664 and 691, 262,088 674 and 861; direct 790 to 1,359)
         const long long cells = teno_t / 4;
         b->teno_shape = cells < 100000 ? 4 : (bl.proof && cells / b->n_cases >= 25000 ? 6 : 8);
         b->prim_stale.assign(b->n_cases, 0);

@@ -825,9 +825,11 @@ void mgpu_ctx::build() {
     const double upd_b = (double)N * (16 + 8 + 32 * 4) + (double)F_flux * 32 * 2;
     stage_bytes = (fo ? 0.0 : recon_bytes) + flux_b + upd_b;
     // the launch shape until mgpu_autotune or a fixed shape says otherwise:
-    // the bulk-copied tables are never slower than the direct kernel and from
-    // 32,768 cells faster (us a launch, shape 7 against 0: 8,192 cells 12.5
-    // and 12.5, 32,768 19 and 31, 524,288 192 and 422)
+    // on thirteen meshes of 512 to 524,288 cells the bulk-copied tables were at
+    // most 0.7 us a launch behind the direct kernel (with a selector, under
+    // 5,000 cells), level to 8,192 cells and ahead from 16,200 (plain form,
+    // shape 7 against 0: 2,048 cells 10.4 and 11.1 us, 16,200 13.2 and 15.2,
+    // 32,768 20 and 32, 524,288 206 and 425)
     if (single() && K == 10) teno_shape = 7;
     lap(6);
     finalized = true;

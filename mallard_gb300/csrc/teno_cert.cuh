@@ -23,7 +23,10 @@
 // the error is under 3 u |d| + 2^-45 max |u|, the last term a perturbation of
 // the data whose effect on sqrt(SI) is max |u| certu.
 // A test that does not prove the decision says nothing: the cell then runs
-// the full kernel.  NaN and infinities prove nothing either.
+// the full kernel.  NaN and infinities prove nothing either: every cell has a
+// directional stencil to compare with (one lacks where its face is a boundary,
+// and a cell with three boundary faces has no neighbours to fill its central
+// stencil from, which the set-up refuses).
 #pragma once
 
 #include "device.h"
