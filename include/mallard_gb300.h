@@ -449,12 +449,16 @@ int mgpu_kernel_times(mgpu_ctx* ctx, double* ms, uint32_t* launches);
  * fastest for later launches.  Until then shape 7 (FP32 form at p = 3): the
  * fastest from 100,000 cells but where a selector is confident nearly
  * everywhere, so a learned run should be tuned on a state of its flow.
- * ms[MGPU_AUTOTUNE_SHAPES] receives the average time per shape (0 where not
+ * ms[n_ms] receives the average times of the first n_ms shapes (0 where not
  * applicable), best the chosen shape.  Both may be NULL.  Other forms have
  * a single shape. */
-#define MGPU_AUTOTUNE_SHAPES 11
+#define MGPU_LAUNCH_SHAPES 11
+int mgpu_autotune_shapes(mgpu_ctx* ctx, double* ms, uint32_t n_ms, int* best);
+/* The same over the first MGPU_AUTOTUNE_SHAPES shapes alone, as this entry was
+ * before there were more: ms holds that many. */
+#define MGPU_AUTOTUNE_SHAPES 8
 int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best);
-/* Fix the reconstruction's launch shape (as mgpu_autotune numbers them);
+/* Fix the reconstruction's launch shape (as mgpu_autotune_shapes numbers them);
  * every shape gives the same results. */
 int mgpu_set_launch_shape(mgpu_ctx* ctx, int shape);
 /* Algorithmic bytes one reconstruction and one full stage move when every

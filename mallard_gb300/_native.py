@@ -25,7 +25,8 @@ BC_TYPES = {"symmetry": 0, "extrapolation": 1, "wall_adiabatic": 2, "upt": 3, "p
 TENO_VARIANTS = {"reference": 0, "corrected": 1, "robust": 2}
 PRECISIONS = {"fp64": 0, "fp64_fast": 1, "fp32": 2}
 VISC_GRADIENTS = {"recon": 0, "green_gauss": 1}
-AUTOTUNE_SHAPES = 11  # MGPU_AUTOTUNE_SHAPES
+AUTOTUNE_SHAPES = 8  # MGPU_AUTOTUNE_SHAPES
+LAUNCH_SHAPES = 11  # MGPU_LAUNCH_SHAPES
 
 TENO_FIELDS = {
     "offsets_stencil_groups": (0, "uint32"),
@@ -132,6 +133,7 @@ def lib():
         "mgpu_probe_conversions": (i32, [i32, vp, vp, vp, vp, C.c_uint64]),
         "mgpu_build_times": (i32, [vp, vp]),
         "mgpu_autotune": (i32, [vp, vp, P(i32)]),
+        "mgpu_autotune_shapes": (i32, [vp, vp, u32, P(i32)]),
         "mgpu_batch_create": (i32, [u32, vp, vp, P(Config), P(vp)]),
         "mgpu_batch_add_boundary": (i32, [vp, u32, i32, vp, i32]),
         "mgpu_batch_finalize": (i32, [vp]),

@@ -252,7 +252,7 @@ namespace f32 {
 // registers, or 256-thread blocks with 64; p = 3 only, other orders use
 // shape 0) or 4..10, forms that copy each tile's table blocks
 // into shared memory with cp.async.bulk; chosen by the autotuner
-constexpr int TENO32_SHAPES = MGPU_AUTOTUNE_SHAPES;
+constexpr int TENO32_SHAPES = MGPU_LAUNCH_SHAPES;
 // cells from which shapes 5-7 are the proof form and 8-10 not the same as 4-6
 constexpr int PROOF_MIN_CELLS = 100000;
 // the batched reconstruction has shape 6, the proof form, and shapes 7 and 8:

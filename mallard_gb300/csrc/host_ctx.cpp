@@ -1250,12 +1250,13 @@ int mgpu_kernel_times(mgpu_ctx* ctx, double* ms, uint32_t* launches) {
     });
 }
 
-int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best) {
+// Times the first `shapes` launch shapes and keeps the fastest.
+static int autotune(mgpu_ctx* ctx, int shapes, double* ms, uint32_t n_ms, int* best) {
     if (int rc = need_ready(ctx)) return rc;
     return guarded([&] {
         // shapes 8-10 are 4-6 again where no proof form takes their place
         const bool proof = ctx->teno.cert && ctx->N >= (uint32_t)f32::PROOF_MIN_CELLS;
-        const int n = !(ctx->single() && ctx->K == 10) ? 1 : (proof ? f32::TENO32_SHAPES : 8);
+        const int n = !(ctx->single() && ctx->K == 10) ? 1 : std::min(shapes, proof ? f32::TENO32_SHAPES : 8);
         std::vector<double> t(f32::TENO32_SHAPES, 0.0);
         cudaEvent_t a, b;
         ck(cudaEventCreate(&a), "cudaEventCreate");
@@ -1292,10 +1293,18 @@ int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best) {
         ctx->teno_shape = choice;
         ctx->drop_graphs();  // recapture with the chosen shape
         if (ms)
-            for (int i = 0; i < f32::TENO32_SHAPES; ++i) ms[i] = t[i];
+            for (uint32_t i = 0; i < n_ms; ++i) ms[i] = i < t.size() ? t[i] : 0.0;
         if (best) *best = choice;
         return MGPU_OK;
     });
+}
+
+int mgpu_autotune_shapes(mgpu_ctx* ctx, double* ms, uint32_t n_ms, int* best) {
+    return autotune(ctx, f32::TENO32_SHAPES, ms, n_ms, best);
+}
+
+int mgpu_autotune(mgpu_ctx* ctx, double* ms, int* best) {
+    return autotune(ctx, MGPU_AUTOTUNE_SHAPES, ms, MGPU_AUTOTUNE_SHAPES, best);
 }
 
 int mgpu_set_launch_shape(mgpu_ctx* ctx, int shape) {

@@ -298,9 +298,9 @@ class Solver:
     def autotune(self):
         """Pick the fastest launch shape of the reconstruction kernel on the
         current state; returns (chosen shape, ms per shape)."""
-        ms = np.zeros(N.AUTOTUNE_SHAPES)
+        ms = np.zeros(N.LAUNCH_SHAPES)
         best = C.c_int()
-        N.check(self._lib.mgpu_autotune(self._h, N.ptr(ms), C.byref(best)))
+        N.check(self._lib.mgpu_autotune_shapes(self._h, N.ptr(ms), len(ms), C.byref(best)))
         return best.value, ms
 
     def set_launch_shape(self, shape):

@@ -2,11 +2,14 @@
 meshes (8-10): the direct kernel's bits with and without a selector, reachable by
 number and by the autotuner."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import mallard_gb300 as mg
 from cases import GAS, four_quadrant
+from mallard_gb300 import _native as N
 from mallard_gb300.selector import Selector, default_weights_path
 from test_gpu_central import shapes_agree, wavy
 
@@ -30,3 +33,8 @@ def test_staged_shapes(n, tuned, learned):
         assert (ms > 0).sum() == tuned and (ms[:tuned] > 0).all() and ms[best] == ms[:tuned].min()
         with pytest.raises(RuntimeError, match="out of range"):
             s.set_launch_shape(11)
+        # the entry that knows eight shapes writes eight times and picks among them
+        eight, first = np.full(11, -1.0), C.c_int(-1)
+        N.check(N.lib().mgpu_autotune(s._h, N.ptr(eight), C.byref(first)))
+        assert (eight[:8] > 0).all() and (eight[8:] == -1.0).all()
+        assert 0 <= first.value < 8 and eight[first.value] == eight[:8].min()
